@@ -112,10 +112,19 @@ __device__ __forceinline__ void aux_deriv_body(const AuxArgs& a, unsigned bx, un
     // a ghost column of a grid off the axis that diff1r leaves unset (all of
     // them in order four, the outermost in order two)
     const bool rg = i < d1r_first(ORD, G.g);
-    const double Dr_gA = rg ? 0.0 : first_difference<ORD>(a.aux[X_GA] + o, 1, i, G.nr, G.g, a.c1r);
-    const double Dz_gB = first_difference<ORD>(a.aux[X_GB] + o, ld, j, G.nz, G.g, a.c1z);
-    const double Dr_gC = rg ? 0.0 : first_difference<ORD>(a.aux[X_GC] + o, 1, i, G.nr, G.g, a.c1r);
-    const double Dz_gC = first_difference<ORD>(a.aux[X_GC] + o, ld, j, G.nz, G.g, a.c1z);
+    double Dr_gA = 0.0, Dz_gB = 0.0, Dr_gC = 0.0, Dz_gC = 0.0;
+    // (one piece of code for all four: it has to stay in the instruction cache)
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+        const bool z = k >= 2;
+        if (!z && rg) continue;
+        const double d = first_difference<ORD>(a.aux[k == 0 ? X_GA : k == 2 ? X_GB : X_GC] + o, z ? ld : 1, z ? j : i,
+                                               z ? G.nz : G.nr, G.g, z ? a.c1z : a.c1r);
+        if (k == 0) Dr_gA = d;
+        else if (k == 1) Dr_gC = d;
+        else if (k == 2) Dz_gB = d;
+        else Dz_gC = d;
+    }
     const double glam = a.aux[X_GLAM][o], gC = a.aux[X_GC][o];
     const double ddr = deldef_r(Dr_gA, Dz_gC, r, glam), ddz = deldef_z(Dr_gC, Dz_gB, r, gC);
     a.aux[X_DELDEFR][o] = ddr;

@@ -50,18 +50,19 @@ __global__ void __launch_bounds__(kWaveThreads) wave_stage_kernel(const __grid_c
         // where the centred stencils and the dissipation of each direction hold
         constexpr int lo = ORD == 2 ? 3 : 4, hi = ORD == 2 ? 2 : 3;
         const bool inr = mi >= lo - g && mi <= nr - hi, inz = mj >= lo - g && mj <= nz - hi;
-        double ur, urr, uzz, uz = 0.0;
-        {
-            const LineSums a = inr ? line_inside<ORD>(u, 1, false)
-                                   : line_edge<ORD>(u, 1, mi < lo - g ? mi - (1 - g) : nr - mi, mi < lo - g, false);
-            ur = sf_scaled(a.d1, a.e, A.C.c1r);
-            urr = sf_scaled(a.d2, a.e2, A.C.c2r);
-        }
-        {
-            const LineSums a = inz ? line_inside<ORD>(u, ld, false)
-                                   : line_edge<ORD>(u, ld, mj < lo - g ? mj - (1 - g) : nz - mj, mj < lo - g, false);
-            if constexpr (PHYS) uz = sf_scaled(a.d1, a.e, A.C.c1z);
-            uzz = sf_scaled(a.d2, a.e2, A.C.c2z);
+        double ur = 0.0, urr = 0.0, uzz = 0.0, uz = 0.0;
+        // (one piece of code for both directions: it has to stay in the
+        // instruction cache)
+#pragma unroll 1
+        for (int dir = 0; dir < 2; ++dir) {
+            const int x = dir ? mj : mi, n = dir ? nz : nr;
+            const long st = dir ? ld : 1;
+            const LineSums a = (dir ? inz : inr) ? line_inside<ORD>(u, st, false, true, false)
+                                                 : line_edge<ORD>(u, st, x < lo - g ? x - (1 - g) : n - x, x < lo - g, false);
+            const double d2 = sf_scaled(a.d2, a.e2, dir ? A.C.c2z : A.C.c2r);
+            const double d1 = PHYS || !dir ? sf_scaled(a.d1, a.e1, dir ? A.C.c1z : A.C.c1r) : 0.0;
+            if (dir) { uz = d1; uzz = d2; }
+            else { ur = d1; urr = d2; }
         }
         double s;
         if constexpr (!PHYS) {
@@ -92,13 +93,11 @@ __global__ void __launch_bounds__(kWaveThreads) wave_stage_kernel(const __grid_c
         // Kreiss-Oliger dissipation on v (dissipation.f90:196-211; order two
         // :121-135)
         sf t = {0, -4000};
-        if (inr) {
-            const LineSums a = line_inside<ORD>(v, 1, true);
-            t = sf_sum(sf_term(t), -(sf_norm(a.nk, a.e) * A.kd));
-        }
-        if (inz) {
-            const LineSums a = line_inside<ORD>(v, ld, true);
-            t = sf_sum(sf_term(t), -(sf_norm(a.nk, a.e) * A.kd));
+#pragma unroll 1
+        for (int dir = 0; dir < 2; ++dir) {
+            if (!(dir ? inz : inr)) continue;
+            const LineSums a = line_inside<ORD>(v, dir ? ld : 1, true, false, false);
+            t = sf_sum(sf_term(t), -(sf_norm63(a.nk, a.ek) * A.kd));
         }
         if (inr || inz) s = s + to_double(t);
         // radiative boundary with unit speed and zero asymptotic value
@@ -107,8 +106,12 @@ __global__ void __launch_bounds__(kWaveThreads) wave_stage_kernel(const __grid_c
         if (mi == nr || mj == nz || (!G.eqsym && mj == 1 - g)) {
             const double r = G.rcol[mi], z = G.zrow[mj];
             const double rr = sqrt(r * r + z * z);
-            s = -(r * first_difference<ORD>(v, 1, mi, nr, g, A.C.c1r) + z * first_difference<ORD>(v, ld, mj, nz, g, A.C.c1z)
-                  + (ld_(v) - 0.0)) / rr;
+            double outward = ld_(v) - 0.0;
+#pragma unroll 1
+            for (int dir = 0; dir < 2; ++dir)
+                outward = fma(dir ? z : r, first_difference<ORD>(v, dir ? ld : 1, dir ? mj : mi, dir ? nz : nr, g,
+                                                                 dir ? A.C.c1z : A.C.c1r), outward);
+            s = -outward / rr;
         }
         double su = ld_(A.v_in + o);  // sell_u = ell_v
         double sv = s;

@@ -12,12 +12,15 @@
 // A number is m * 2^e with a signed 64-bit mantissa, normalised to
 // 2^61 <= |m| < 2^62 (the unnormalised rest of a cancellation and zero have a
 // smaller |m|).  Multiplication and addition are the schoolbook algorithms on
-// mantissas and exponents; a product is cut, not rounded, at 2^-57 of its
-// value or below, a sum at 2^-58 of its largest term, so each operation is
-// nearer to the exact result than a correctly rounded FP64 one (2^-53) can be
-// relied on to be.  Exponents of inputs near the ends of the FP64 range are
-// not trapped: results below the normal range become zero, results above it
-// NaN.
+// mantissas and exponents.  A product of normalised numbers is cut, not
+// rounded, at 2.25 * 2^-58 of its value, a sum at 2^-58 of its largest term:
+// both are nearer to the exact result than a correctly rounded FP64 operation
+// (2^-53) can be relied on to be.  What is left of a cancellation of more than
+// 30 bits is moved up by 29, so a product of it is cut at 2^-86 of what the
+// product of the terms before the cancellation would have been.
+//
+// Results below the normal range are subnormal, results above it infinite;
+// a NaN or an infinity among the inputs makes the result NaN.
 #pragma once
 #include <stdint.h>
 #include <string.h>
@@ -48,6 +51,16 @@ OLLIN_HD unsigned long long sf_shr_u(unsigned long long m, unsigned n) {
     return r;
 #else
     return n > 63u ? 0ull : m >> n;
+#endif
+}
+
+OLLIN_HD unsigned long long sf_shl_u(unsigned long long m, unsigned n) {
+#if defined(__CUDA_ARCH__)
+    unsigned long long r;
+    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(m), "r"(n));
+    return r;
+#else
+    return n > 63u ? 0ull : m << n;
 #endif
 }
 
@@ -104,13 +117,27 @@ OLLIN_HD sf sf_norm(long long m, int e) {
     return {(long long)((unsigned long long)m << s), e - (int)s};
 }
 
+// the same for |m| < 2^63
+OLLIN_HD sf sf_norm63(long long m, int e) {
+    unsigned s = sf_lead((int)(m >> 32));
+    s = s < 31u ? s : 31u;
+    return {(long long)((unsigned long long)m << (s - 1u)) >> 1, e + 2 - (int)s};
+}
+
 OLLIN_HD sf to_sf(double x) {
     const unsigned long long b = sf_bits(x);
     const int e = (int)(b >> 52) & 0x7ff;
-    unsigned long long a = ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 9;
-    if (e == 0) a = 0;  // zero and subnormal numbers
+    const unsigned long long a = ((b & 0x000fffffffffffffull) | (e == 0 ? 0 : 0x0010000000000000ull)) << 9;
     const long long s = (long long)b >> 63;
-    return {(long long)(a ^ (unsigned long long)s) - s, e == 0x7ff ? kSfNaN : e - 1084};
+    return {(long long)(a ^ (unsigned long long)s) - s, e == 0x7ff ? kSfNaN : (e == 0 ? 1 : e) - 1084};
+}
+
+// The magnitude bits of a result outside the normal range: 1.f with f below
+// the highest bit of a, bit 63, and the biased exponent x + 1.  Infinity above
+// the range, NaN for kSfNaN, and below it the nearest subnormal number.
+OLLIN_HD unsigned long long sf_outside(unsigned long long a, int x) {
+    if (x > 0) return x > kSfNaN / 2 ? 0x7ff8000000000000ull : 0x7ff0000000000000ull;
+    return (sf_shr_u(a, (unsigned)(10 - x)) + 1) >> 1;
 }
 
 // the nearest double of m * 2^e
@@ -118,12 +145,11 @@ OLLIN_HD double to_double(long long m, int e) {
     const long long s = m >> 63;
     unsigned long long a = (unsigned long long)((m ^ s) - s);
     const int z = sf_clz64(a);
-    a = (a << (z & 63)) >> 1;                 // highest bit at 62
-    int x = e + 1085 - z;                     // biased exponent of 1.f, less one: the kept bit 52 adds it
-    a = (a + 0x200ull) >> 10;
-    unsigned long long r = ((unsigned long long)(unsigned)x << 52) + a;
-    if (x < 0 || m == 0) r = 0;
-    if (x >= 0x7fe) r = 0x7ff8000000000000ull;
+    a <<= z & 63;
+    const int x = e + 1085 - z;               // biased exponent of 1.f, less one: the kept bit 52 adds it
+    unsigned long long r = ((unsigned long long)(unsigned)x << 52) + ((a >> 11) + ((a >> 10) & 1));
+    if ((unsigned)x >= 0x7feu) r = sf_outside(a, x);
+    if (m == 0 && e < kSfNaN / 2) r = 0;
     return sf_from_bits(r | ((unsigned long long)s & 0x8000000000000000ull));
 }
 OLLIN_HD double to_double(sf a) { return to_double(a.m, a.e); }
@@ -166,8 +192,8 @@ OLLIN_HD double sf_scaled(long long n, int e, sfc c) {
     p <<= k;
     const int x = e + c.e + 1149 - z - k;
     unsigned long long r = ((unsigned long long)(unsigned)x << 52) + ((p >> 11) + ((p >> 10) & 1));
-    if (x < 0 || a == 0) r = 0;
-    if (x >= 0x7fe) r = 0x7ff8000000000000ull;
+    if ((unsigned)x >= 0x7feu) r = sf_outside(p, x);
+    if (a == 0) r = 0;
     return sf_from_bits(r | ((unsigned long long)s & 0x8000000000000000ull));
 }
 
@@ -188,35 +214,100 @@ OLLIN_HD sf sf_sum(sfp a, sfp b, sfp c, sfp d) {
     return sf_norm(sf_shr(a.m, e - a.e) + sf_shr(b.m, e - b.e) + (sf_shr(c.m, e - c.e) + sf_shr(d.m, e - d.e)), e);
 }
 
-// N neighbouring values as integers in one unit, 2^(e - G) of the returned e
-// = (largest exponent) - 1075: every value whose exponent is within G of the
-// largest is exact, the others are cut at that unit.  With G = 2 a sum with
-// integer weights of total 128 stays below 2^62, with G = 0 one of total 512.
-// A NaN or an infinity among them makes every weighted sum NaN.
+// N neighbouring values as integers in one unit, 2^e of e = (largest exponent)
+// - 1075 - G: every value whose exponent is within G of the largest is exact,
+// the others are cut at that unit.  With G = 4 a sum with integer weights of
+// total 64 stays below 2^63, with G = 2 one of total 128 below 2^62.  ``top``:
+// the largest exponent, as bits of the high word.  True if every value is exact
+// (zeros too); false otherwise, and for values that sf_spread has more to say
+// about.
 template <int G, int N>
-OLLIN_HD int sf_align(const unsigned long long (&b)[N], long long (&m)[N]) {
-    int top = 0;
+OLLIN_HD bool sf_align_fast(const unsigned long long (&b)[N], long long (&m)[N], int& e, int& top) {
+    int t = 0;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         const int x = (int)(b[k] >> 32) & 0x7ff00000;
-        top = x > top ? x : top;
+        t = x > t ? x : t;
     }
+    // the smallest distance from the largest exponent beyond G; zeros lie 128
+    // and more away, values within G wrap around
+    unsigned beyond = ~0u;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-        const unsigned n = (unsigned)(top - ((int)(b[k] >> 32) & 0x7ff00000)) >> 20;
+        const unsigned d = (unsigned)(t - ((int)(b[k] >> 32) & 0x7ff00000));
+        beyond = d - ((G + 1) << 20) < beyond ? d - ((G + 1) << 20) : beyond;
         unsigned long long a = ((b[k] & 0x000fffffffffffffull) | 0x0010000000000000ull) << G;
-        a = sf_shr_u(a, n);
+        a = sf_shr_u(a, d >> 20);
         const long long s = (long long)b[k] >> 63;
         m[k] = (long long)(a ^ (unsigned long long)s) - s;
     }
-    // NaN or infinity; only numbers below 2^-958 (zeros of either sign among
-    // them), which count as zero
+    top = t;
+    e = (t >> 20) - 1075 - G;
+    const bool plain = (unsigned)(t - (128 << 20)) < (unsigned)(0x7ff00000 - (128 << 20));
+    return plain && beyond >= (unsigned)((128 - (G + 1)) << 20);
+}
+
+// Values that are not all exact: 0 if they are all zero, 1 if sf_rest gives what
+// was cut off, 2 if they are too far apart for that (by more than G + kSfRest in
+// their exponents), too small (below 2^-895) or not finite.
+constexpr int kSfRest = 21;
+template <int G, int N>
+OLLIN_HD int sf_spread(const unsigned long long (&b)[N], int top) {
+    if ((unsigned)(top - (128 << 20)) >= (unsigned)(0x7ff00000 - (128 << 20))) {
+        unsigned long long any = 0;
+#pragma unroll
+        for (int k = 0; k < N; ++k) any |= b[k] << 1;
+        return any == 0 ? 0 : 2;
+    }
+    unsigned far = 0;  // the largest distance of one that is not zero
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const unsigned h = (unsigned)(b[k] >> 32) & 0x7ff00000u, d = h == 0 ? 0u : (unsigned)top - h;
+        far = d > far ? d : far;
+    }
+    return far <= (unsigned)((G + kSfRest) << 20) ? 1 : 2;
+}
+
+// Keeps the compiler from running what follows, which is rarely needed, in
+// advance of the branch that leads to it.
+OLLIN_HD void sf_rare() { asm volatile("" ::: "memory"); }
+
+// N values as by sf_align_fast, for a caller that takes them cut: zero if they
+// are all below 2^-958, and such that every weighted sum is NaN if one of them
+// is a NaN or an infinity.
+template <int G, int N>
+OLLIN_HD int sf_align(const unsigned long long (&b)[N], long long (&m)[N]) {
+    int e, top;
+    sf_align_fast<G>(b, m, e, top);
     if (top == 0x7ff00000 || top < (64 << 20)) {
 #pragma unroll
         for (int k = 0; k < N; ++k) m[k] = top == 0x7ff00000 ? 1ll << (4 * k + 8) : 0;
         return top == 0x7ff00000 ? kSfNaN : -1200;
     }
-    return (top >> 20) - 1075 - G;
+    return e;
+}
+
+// What was cut off the aligned values: kSfRest more bits of each, in units of
+// 2^(e - kSfRest), with the sign of the value.  Sums with integer weights of
+// total 640 fit in 32 bits.
+template <int G, int N>
+OLLIN_HD void sf_rest(const unsigned long long (&b)[N], int top, int (&r)[N]) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const unsigned n = (unsigned)(top - ((int)(b[k] >> 32) & 0x7ff00000)) >> 20;
+        // the bits below bit n of the mantissa with its G zeros, bit n - 1 first
+        const unsigned long long a = ((b[k] & 0x000fffffffffffffull) | 0x0010000000000000ull) << G;
+        const unsigned q = (unsigned)(sf_shl_u(a, (unsigned)(64 - (int)n)) >> (64 - kSfRest));
+        r[k] = (long long)b[k] < 0 ? -(int)q : (int)q;
+    }
+}
+// a weighted sum n of the aligned values and the same sum c of their rests as
+// one integer; ``lift``: by how much its unit is smaller
+OLLIN_HD long long sf_join(long long n, int c, int& lift) {
+    int s = sf_clz64((unsigned long long)(n ^ (n >> 63))) - 2;
+    s = s < 0 ? 0 : (s < kSfRest ? s : kSfRest);
+    lift = s;
+    return (long long)((unsigned long long)n << s) + (c >> (kSfRest - s));
 }
 
 }  // namespace ollin
