@@ -43,9 +43,15 @@ __device__ __forceinline__ void aux_point_body(const AuxArgs& a, unsigned bx, un
         // rcbrt, and A + A d is rounded once.
         const double rc = r * C;
         const double x = fma(fma(A, B, -(rc * rc)), H, -1.0);  // hdet = 1
-        double d = x * fma(x, fma(x, fma(x, fma(x, -91.0 / 729.0, 35.0 / 243.0), -14.0 / 81.0), 2.0 / 9.0), -1.0 / 3.0);
-        if (!(fabs(x) < 0x1p-9)) d = rcbrt((A * B - rc * rc) * H) - 1.0;
-        A = fma(A, d, A); B = fma(B, d, B); C = fma(C, d, C); H = fma(H, d, H);
+        // Elsewhere d says too little of a det^(-1/3) well below 1 (eight
+        // digits are lost at det = 10^24): the factor itself is taken.
+        if (fabs(x) < 0x1p-9) {
+            const double d = x * fma(x, fma(x, fma(x, fma(x, -91.0 / 729.0, 35.0 / 243.0), -14.0 / 81.0), 2.0 / 9.0), -1.0 / 3.0);
+            A = fma(A, d, A); B = fma(B, d, B); C = fma(C, d, C); H = fma(H, d, H);
+        } else {
+            const double q = rcbrt((A * B - rc * rc) * H);
+            A *= q; B *= q; C *= q; H *= q;
+        }
         a.st[F_A][o] = A; a.st[F_B][o] = B; a.st[F_C][o] = C; a.st[F_H][o] = H;
     }
     const double gA = B * H, gB = A * H, gH = 1.0 / H, gC = -C * H;
