@@ -22,11 +22,10 @@
 #include <mutex>
 #include <string>
 #include <unordered_map>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "../../include/ollin_gpu.h"
+#include "parallel_rows.h"
 #include "ollin_kernels.h"
 
 using namespace ollin;
@@ -2040,30 +2039,6 @@ int mixed_elliptic(ollin_handle* h, WaveSolve& S) {
     }
     return OLLIN_OK;
 }
-
-// f(j) for the rows lo <= j < hi, on several host threads where there are
-// points enough (the initial data take about 50 ns a point in exp, log and
-// pow).  Rows are independent, so the values do not depend on the threads.
-template <typename F>
-void parallel_rows(int lo, int hi, size_t points, const F& f) {
-    const size_t most = std::min<size_t>(16, std::max(1u, std::thread::hardware_concurrency()));
-    const int n = (int)std::min<size_t>(most, points / 32768 + 1);
-    auto part = [&](int k) {
-        for (int j = lo + (int)((long)(hi - lo) * k / n); j < lo + (int)((long)(hi - lo) * (k + 1) / n); ++j) f(j);
-    };
-    std::vector<std::thread> threads;
-    threads.reserve(n);
-    int k = 1;
-    try {
-        for (; k < n; ++k) threads.emplace_back(part, k);
-    } catch (const std::system_error&) {
-        // no more threads to be had: the rest of the rows here
-    }
-    part(0);
-    for (; k < n; ++k) part(k);
-    for (std::thread& t : threads) t.join();
-}
-
 
 // The pre-solve part of the elliptic initial data, the solve, and the
 // solution of every level copied to the host (``ell_u``, all points).
