@@ -23,7 +23,7 @@ multivariate Horner form, common subexpressions) and emits CUDA.
 import sympy as sp
 
 INPUTS = [
-    "r", "ir", "alpha", "chi", "Ac", "Bc", "Hc", "Cc", "trK", "kA", "kB", "kC", "kH",
+    "r", "ir", "alpha", "Ac", "Bc", "Hc", "Cc", "trK", "kA", "kB", "kC", "kH",
     "Dlr", "Dlz", "gA", "gB", "gH", "gC", "lam", "Alam", "glam", "DDr", "DDz", "ipsi4", "eta",
     "da_r", "da_z", "da_rr", "da_zz", "da_rz", "dan_r", "dan_z",
     "dA_r", "dA_z", "dA_rr", "dA_zz", "dA_rz",
@@ -36,23 +36,23 @@ INPUTS = [
 ]
 
 # The algebra is cut into tasks that the warps of a block run side by side on
-# the same points: each task's outputs are temporaries (``let``) or sources.
-# The last combinations (Ricci scalar, sources of trK, KTA, KTB, KTC and the
-# Hamiltonian constraint) need several tasks' outputs and stand in the kernel.
-TASKS = {
-    # all of the sources at once, and the Hamiltonian constraint, for one warp
-    "sources": ["s_trK", "s_KTA", "s_KTB", "s_KTC", "s_Dlr", "s_Dlz"],
-    "ham": ["ham", "RSCAL"],
-    "lapse": ["D2A", "D2B", "D2C", "Lapla_alpha"],
-    "curvature": ["KT2_A", "KT2_B", "KT2_C", "KT2"],
-    "ricci_phi": ["PA", "PB", "PH", "PC"],
-    "ricci_ab": ["QA", "QB"],
-    "ricci_ch": ["QC", "QH"],
-    "delta_r": ["s_Dlr"],
-    "delta_z": ["s_Dlz"],
-    "mom_r": ["mom_r"],
-    "mom_z": ["mom_z"],
-}
+# the same points, or one warp after one another: each task's outputs are
+# temporaries (``let``) or sources.  The tasks of a group share their common
+# subexpressions.  The last combinations (Ricci scalar, sources of trK, KTA,
+# KTB, KTC and the Hamiltonian constraint) need several tasks' outputs and
+# stand in the kernel.
+GROUPS = [
+    {
+        "lapse": ["D2A", "D2B", "D2C", "Lapla_alpha"],
+        "curvature": ["KT2_A", "KT2_B", "KT2_C", "KT2"],
+        "ricci_phi": ["PA", "PB", "PH", "PC"],
+        "ricci_ab": ["QA", "QB"],
+        "ricci_ch": ["QC", "QH"],
+        "delta_r": ["s_Dlr"],
+        "delta_z": ["s_Dlz"],
+    },
+    {"mom_r": ["mom_r"], "mom_z": ["mom_z"]},
+]
 
 
 def algebra(x, let):
@@ -163,10 +163,7 @@ def algebra(x, let):
     QB = let("QB", RB)
     QH = let("QH", RH)
     QC = let("QC", RC)
-    RA, RB, RH, RC = QA + PA, QB + PB, QH + PH, QC + PC
-    RSCAL = let("RSCAL", (gA * RA + gB * RB + gH * RH + two * r2 * gC * RC) * ipsi4)
 
-    # R_ij = Q_ij + P_ij; the Ricci scalar (:1483-1493)
     # traceless curvature contractions (:944-1031)
     KT_up_rr = let("KT_up_rr", (2 * gA * gC * kC + gC ** 2 * kB) * r2 + gA ** 2 * kA)
     KT_up_zz = let("KT_up_zz", (gC ** 2 * kA + 2 * gC * gB * kC) * r2 + gB ** 2 * kB)
@@ -175,7 +172,6 @@ def algebra(x, let):
     KT2_B = let("KT2_B", (kC ** 2 * gA + 2 * kC * gC * kB) * r2 + gB * kB ** 2)
     KT2_C = let("KT2_C", kC ** 2 * gC * r2 + kA * gA * kC + kA * gC * kB + kC * gB * kB)
     KT2 = let("KT2", gA * KT2_A + gB * KT2_B + gH * kH ** 2 * gH + two * gC * KT2_C * r2)
-    K2 = KT2 + third * trK ** 2
 
     # divergence of KT (calc_DIVKTA.f90, non-angmom)
     dkAr, dkAz, dkBr, dkBz, dkCr, dkCz = x.Dr_KTA, x.Dz_KTA, x.Dr_KTB, x.Dz_KTB, x.Dr_KTC, x.Dz_KTC
@@ -228,12 +224,7 @@ def algebra(x, let):
     DIVA_KT_z = let("DIVA_KT_z", DIVA_KT_z)
 
     # sources without shift and matter terms (sources_geometry.f90)
-    trterm = let("trterm", -Lapla + alpha * RSCAL)
     out = {}
-    out["s_trK"] = -Lapla + alpha * K2
-    out["s_KTA"] = alpha * (trK * kA - two * KT2_A) + (-D2A + alpha * RA) * ipsi4 - third * Ac * trterm
-    out["s_KTB"] = alpha * (trK * kB - two * KT2_B) + (-D2B + alpha * RB) * ipsi4 - third * Bc * trterm
-    out["s_KTC"] = alpha * (trK * kC - two * KT2_C) + (-D2C + alpha * RC) * ipsi4 - third * Cc * trterm
     # the lapse gradient of the Delta sources is the one maximalslicing.f90
     # recomputes (dan_*); D2cov_alpha and Lapla_alpha above keep the values of
     # the last ``auxiliary`` call (da_*); the two differ only in the first
@@ -242,11 +233,7 @@ def algebra(x, let):
         + x.eta * alpha * (DIV_KT_r + six * (KT_up_rr * Dr_phi + KT_up_rz * Dz_phi) - two * third * (gA * x.Dr_trK + r * gC * x.Dz_trK))
     out["s_Dlz"] = -two * (KT_up_rz * x.dan_r + KT_up_zz * x.dan_z) - two * alpha * DIVA_KT_z \
         + x.eta * alpha * (DIV_KT_z + six * (KT_up_rz * Dr_phi + KT_up_zz * Dz_phi) - two * third * (r * gC * x.Dr_trK + gB * x.Dz_trK))
-    # constraints (constraints.f90:55-149), vacuum part
-    out["ham"] = RSCAL - KT2 + two * third * trK ** 2
+    # momentum constraints (constraints.f90:55-149), vacuum part
     out["mom_r"] = DIV_KT_r + six * (KT_up_rr * Dr_phi + KT_up_rz * Dz_phi) - two * third * (gA * x.Dr_trK + r * gC * x.Dz_trK)
     out["mom_z"] = DIV_KT_z + six * (KT_up_rz * Dr_phi + KT_up_zz * Dz_phi) - two * third * (r * gC * x.Dr_trK + gB * x.Dz_trK)
-    out["RSCAL"] = RSCAL
-    out["KT2"] = KT2
-    out["Lapla_alpha"] = Lapla
     return out

@@ -8,9 +8,13 @@ reference's Maple-generated monomial sums:
     coefficient is put in multivariate Horner form with the variables ordered
     by how many monomials they occur in (the cheapest of a few orderings under
     an FMA-aware cost model is kept);
-  * common subexpressions across all temporaries are then shared;
-  * the result is printed as straight-line CUDA with products written so
-    that nvcc contracts the additions into FMAs.
+  * common subexpressions across all temporaries of a group of tasks are then
+    shared;
+  * the result is printed as straight-line CUDA, a function per task with what
+    its outputs need.  Every rounding is written out (fma, and products and
+    sums that the compiler may not contract): a warp that runs several tasks
+    forms their common subexpressions once, warps that run one task each form
+    them again, and both get the same bits.
 Every rewritten temporary is checked to be algebraically identical to the
 spec expression before it is emitted.
 
@@ -20,7 +24,6 @@ import os
 import sys
 
 import sympy as sp
-from sympy.printing.c import C99CodePrinter
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, HERE)
@@ -110,30 +113,70 @@ def optimise(expr, r, ir):
     return best
 
 
-class CudaPrinter(C99CodePrinter):
-    def _print_Pow(self, expr):
-        b, k = expr.args
-        k = int(k)
-        base = self.parenthesize(b, 100)
-        if k == 2:
-            return "(%s * %s)" % (base, base)
-        if k == 3:
-            return "(%s * %s * %s)" % (base, base, base)
-        if k == 4:
-            return "((%s * %s) * (%s * %s))" % (base, base, base, base)
-        raise ValueError("power %d" % k)
-
-    def _print_Rational(self, expr):
-        return "%s" % repr(float(expr.p) / float(expr.q)) if expr.q != 1 else "%d.0" % expr.p
-
-    def _print_Integer(self, expr):
-        return "%d.0" % int(expr)
-
-    def _print_Float(self, expr):
-        return repr(float(expr))
+def number(q):
+    return "%d.0" % q.p if q.q == 1 else repr(float(q.p) / float(q.q))
 
 
-def generate(outputs):
+def factors(e):
+    """The factors of a product, powers multiplied out, without its sign."""
+    out = []
+    for f in e.args if e.is_Mul else (e,):
+        if f.is_Pow:
+            k = int(f.args[1])
+            if k == 4:
+                out += [sp.Pow(f.args[0], 2, evaluate=False)] * 2
+            elif k in (2, 3):
+                out += [f.args[0]] * k
+            else:
+                raise ValueError("power %d" % k)
+        elif not (f.is_Number and abs(f) == 1):
+            out.append(abs(f) if f.is_Number else f)
+    return out
+
+
+def negative(e):
+    return e.is_Number and e < 0 or e.is_Mul and e.args[0].is_Number and e.args[0] < 0
+
+
+def product(fs):
+    return " * ".join(text(f, True) for f in fs)
+
+
+def text(e, inner=False):
+    """``e`` in CUDA with its roundings: sums of products as chains of fma."""
+    if e.is_Symbol:
+        return e.name
+    if e.is_Number:
+        t = number(e)
+        return "(%s)" % t if inner and e < 0 else t
+    if e.is_Mul or e.is_Pow:
+        if e.is_Pow and int(e.args[1]) == 2:
+            b = text(e.args[0], True)
+            t = "%s * %s" % (b, b)
+        else:
+            t = ("-" if negative(e) else "") + product(factors(e))
+        return "(%s)" % t if inner else t
+    if e.is_Add:
+        single = [t for t in e.args if len(factors(t)) == 1]
+        products = [t for t in e.args if len(factors(t)) > 1]
+        if single:
+            single.sort(key=lambda t: (bool(negative(t)), str(t)))
+            acc = ("-" if negative(single[0]) else "") + text(factors(single[0])[0], True)
+            for t in single[1:]:
+                acc += (" - " if negative(t) else " + ") + text(factors(t)[0], True)
+        else:
+            t, products = products[0], products[1:]
+            acc = ("-" if negative(t) else "") + product(factors(t))
+        for t in products:
+            fs = factors(t)
+            acc = "fma(%s(%s), %s, %s)" % ("-" if negative(t) else "", product(fs[:-1]), text(fs[-1]), acc)
+        return "(%s)" % acc if inner and not products else acc
+    raise ValueError(str(e))
+
+
+def group(outputs):
+    """The temporaries and outputs of a group of tasks, optimised together:
+    definitions, the outputs' expressions, and the instruction counts."""
     syms = {n: sp.Symbol(n) for n in bssn_spec.INPUTS}
 
     class X:
@@ -150,7 +193,7 @@ def generate(outputs):
 
     outs = bssn_spec.algebra(x, let)
     letmap = dict(lets)
-    exprs = [outs[o] if o in outs and o not in ("Lapla_alpha", "KT2") else letmap[sp.Symbol("t_" + o)] for o in outputs]
+    exprs = [outs[o] if o in outs else letmap[sp.Symbol("t_" + o)] for o in outputs]
     # the temporaries these outputs need; an output that another one uses is
     # one of them
     need, stack = set(), list(exprs)
@@ -167,46 +210,46 @@ def generate(outputs):
     # common subexpressions across everything
     repl, reduced = sp.cse([e for _, e in opt] + oexp, symbols=sp.numbered_symbols("c"), optimizations="basic")
     after = sum(cost(e) for _, e in repl) + sum(cost(e) for e in reduced)
-    # Emission order: depth-first from each output, every definition placed
-    # just before its first use, so that temporaries live briefly (the
-    # register pressure of the straight-line code follows the text order).
     defs = dict(list(repl) + [(s, e) for (s, _), e in zip(opt, reduced[:len(opt)])])
-    used, emitted, order = set(), set(syms.values()), []
+    return defs, dict(zip(outputs, reduced[len(opt):])), before, after
+
+
+def task(defs, exprs, outputs):
+    """The lines of one task.  Emission order: depth-first from each output,
+    every definition placed just before its first use, so that temporaries
+    live briefly (the register pressure of the straight-line code follows the
+    text order)."""
+    used, emitted, lines, count = set(), set(), [], 0
 
     def emit(sym):
-        if sym in emitted:
+        nonlocal count
+        if sym in emitted or sym not in defs:
             return
         for dep in sorted(defs[sym].free_symbols, key=lambda q: q.name):
             emit(dep)
-        order.append((sym, defs[sym]))
+        lines.append("    const double %s = %s;" % (sym, text(defs[sym])))
+        used.update(defs[sym].free_symbols)
+        count += cost(defs[sym])
         emitted.add(sym)
 
-    results = []
-    for o, e in zip(outputs, reduced[len(opt):]):
-        for dep in sorted(e.free_symbols, key=lambda q: q.name):
+    for o in outputs:
+        for dep in sorted(exprs[o].free_symbols, key=lambda q: q.name):
             emit(dep)
-        results.append((o, e))
-    for _, e in order + results:
-        used |= e.free_symbols
-    inputs = [n for n in bssn_spec.INPUTS if syms[n] in used]
-    return inputs, order, results, before, after
-
-
-def body_double(inputs, order, results):
-    pr = CudaPrinter()
-    lines = ["    const double %s = in.%s;" % (n, n) for n in inputs]
-    lines += ["    const double %s = %s;" % (s, pr.doprint(e)) for s, e in order]
-    lines += ["    o_%s = %s;" % (o, pr.doprint(e)) for o, e in results]
-    return lines
+        lines.append("    o_%s = %s;" % (o, text(exprs[o])))
+        used.update(exprs[o].free_symbols)
+        count += cost(exprs[o])
+    names = set(s.name for s in used)
+    return ["    const double %s = in.%s;" % (n, n) for n in bssn_spec.INPUTS if n in names] + lines, count
 
 
 HEADER = """// Generated by csrc/gen/gen_rhs.py from csrc/gen/bssn_spec.py -- do not edit.
 //
 // Pointwise BSSN algebra (lapse Laplacian, Ricci tensor, traceless-curvature
 // contractions, divergence of KT, geometric sources and constraints) in an
-// FP64-instruction-minimised form, cut into the tasks that the warps of a
-// block run side by side.  Estimated FP64 instructions per point
-// (FMA-contracted), as written in the spec -> here:
+// FP64-instruction-minimised form, cut into tasks that one warp runs after one
+// another or the warps of a block side by side, with the same bits.  Estimated
+// FP64 instructions per point (FMA-contracted): of a group of tasks as written
+// in the spec -> with all its common subexpressions, and of each task alone:
 %(costs)s
 #pragma once
 
@@ -223,17 +266,20 @@ struct AlgIn {
 
 def main():
     costs, bodies = [], []
-    for task, outputs in bssn_spec.TASKS.items():
-        inputs, order, results, before, after = generate(outputs)
-        costs.append("//   %-10s %4d -> %d" % (task, before, after))
-        bodies.append("__device__ __forceinline__ void alg_%s(const AlgIn& in, %s) {\n%s\n}\n" % (
-            task, ", ".join("double& o_" + o for o in outputs), "\n".join(body_double(inputs, order, results))))
-    text = HEADER % dict(costs="\n".join(costs), inputs=", ".join(bssn_spec.INPUTS), bodies="\n".join(bodies))
-    out = os.path.join(os.path.dirname(HERE), "rhs_algebra_gen.cuh")
-    with open(out, "w") as f:
-        f.write(text)
+    for tasks in bssn_spec.GROUPS:
+        defs, exprs, before, after = group(sum(tasks.values(), []))
+        costs.append("//   %4d -> %d" % (before, after))
+        for name, outputs in tasks.items():
+            lines, count = task(defs, exprs, outputs)
+            costs.append("//     %-10s %4d" % (name, count))
+            bodies.append("__device__ __forceinline__ void alg_%s(const AlgIn& in, %s) {\n%s\n}\n" % (
+                name, ", ".join("double& o_" + o for o in outputs), "\n".join(lines)))
+    out = HEADER % dict(costs="\n".join(costs), inputs=", ".join(bssn_spec.INPUTS), bodies="\n".join(bodies))
+    path = os.path.join(os.path.dirname(HERE), "rhs_algebra_gen.cuh")
+    with open(path, "w") as f:
+        f.write(out)
     print("\n".join(costs))
-    print("wrote", out)
+    print("wrote", path)
 
 
 if __name__ == "__main__":

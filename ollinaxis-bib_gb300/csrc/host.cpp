@@ -14,6 +14,7 @@
 // state at the start of the current (p) and previous (pp) step, so it is read
 // straight from those slots.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -33,6 +34,9 @@ using namespace ollin;
 namespace ollin {
 thread_local bool g_chain_launch = false;
 thread_local LaunchRecorder* g_recorder = nullptr;
+// evolutions of the process with a step under way (queued or being issued): a
+// measure of the GPU's load, by which a step takes the kernels that suit it
+std::atomic<int> g_stepping{0};
 
 static std::unordered_map<const void*, MultiLaunchFn>& multi_registry() {
     static std::unordered_map<const void*, MultiLaunchFn> m;
@@ -141,6 +145,8 @@ struct ollin_handle {
     long long launches = 0;
     bool initialized = false;
     bool step_queued = false;  // ollin_gpu_step_begin ran, ollin_gpu_step_end not yet
+    int sms = 1;               // SMs of the device
+    int beside = 1;            // evolutions being stepped, this one included, when its step was issued
     // ollin_gpu_step_graphs: a coarse step is captured and replayed as one
     // graph launch (the executable graph is updated in place each step)
     bool graphs = false;
@@ -506,6 +512,10 @@ StageArgs stage_args(ollin_handle* h, DLevel& L, int in_slot, int out_slot, bool
     }
     a.t0 = L.last_aux_t0 ? 1 : 0;
     a.deldef = L.deldef ? 1 : 0;
+    a.sms = h->sms;
+    a.beside = h->beside;
+    // kernels launched one by one go through eight queues, whatever their streams
+    a.abreast = g_recorder || (h->graphs && !h->ktime) ? h->beside : std::min(h->beside, 8);
     a.evolve_phi = t0 ? 1 : 0;
     a.level0 = L.level == 0;
     // sources_shift.f90:43 reads the time of box 0's level 0 when the stage runs
@@ -1040,6 +1050,7 @@ int analysis(ollin_handle* h, int level, int what) {
     DLevel& L = h->L[level];
     StageArgs a = stage_args(h, L, L.cur, L.cur, L.last_aux_t0);
     a.analysis = what;
+    a.beside = a.abreast = 1;
     launch_stage_rhs(a, h->stream);
     int rc = after_launch(h);
     if (rc) return rc;
@@ -2393,6 +2404,12 @@ int ollin_gpu_create(const ollin_params* p, ollin_handle** out) {
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
         return fail(OLLIN_ECUDA, "no CUDA device is available");
     auto* h = new ollin_handle();
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        delete h;
+        return fail(OLLIN_ECUDA, "the device cannot be queried");
+    }
     h->P = *p;
     h->g = ghost_zones(*p);
     h->shift = p->shift != OLLIN_SHIFT_NONE;
@@ -2448,6 +2465,7 @@ int ollin_gpu_create(const ollin_params* p, ollin_handle** out) {
 void ollin_gpu_destroy(ollin_handle* h) {
     if (!h) return;
     if (h->stream) cudaStreamSynchronize(h->stream);
+    if (h->step_queued) --g_stepping;
     for (DLevel& L : h->L) {
         if (L.pool) cudaFree(L.pool);
         if (L.ptab) cudaFree(L.ptab);
@@ -2791,9 +2809,21 @@ int ollin_gpu_aux(ollin_handle* h, int level) {
     return OLLIN_OK;
 }
 
+namespace {
+// n evolutions' steps are under way as long as this lives
+struct Stepping {
+    int n, beside;
+    explicit Stepping(int k) : n(k), beside(g_stepping += k) {}
+    ~Stepping() { g_stepping -= n; }
+    Stepping(const Stepping&) = delete;
+};
+}  // namespace
+
 int ollin_gpu_coarse_step(ollin_handle* h, double* t_out) {
     if (!h) return fail(OLLIN_EINVAL, "null handle");
     if (!h->initialized) return fail(OLLIN_ESTATE, "ollin_gpu_initialize must run before the first step");
+    Stepping stepping(1);
+    h->beside = stepping.beside;
     g_chain_launch = h->chain;
     int rc = h->graphs && !h->ktime ? captured_step(h) : onestep(h, 0);
     g_chain_launch = false;
@@ -2852,6 +2882,7 @@ int ollin_gpu_step_begin(ollin_handle* h) {
     if (!h) return fail(OLLIN_EINVAL, "null handle");
     if (!h->initialized) return fail(OLLIN_ESTATE, "ollin_gpu_initialize must run before the first step");
     if (h->step_queued) return fail(OLLIN_ESTATE, "a step is already queued on this handle");
+    h->beside = ++g_stepping;
     g_chain_launch = h->chain;
     int rc = h->graphs && !h->ktime ? captured_step(h) : onestep(h, 0);
     g_chain_launch = false;
@@ -2883,6 +2914,7 @@ int ollin_gpu_step_end(ollin_handle* h, double* t_out) {
     if (!h) return fail(OLLIN_EINVAL, "null handle");
     if (!h->step_queued) return fail(OLLIN_ESTATE, "no step is queued on this handle");
     h->step_queued = false;
+    --g_stepping;
     unsigned int flag = 0;
     CUDA_OR_FAIL(cudaMemcpyAsync(&flag, h->d_flag, sizeof(flag), cudaMemcpyDeviceToHost, h->stream));
     CUDA_OR_FAIL(cudaStreamSynchronize(h->stream));
@@ -2935,7 +2967,9 @@ int ollin_gpu_coarse_step_many(ollin_handle* const* hs, int n, double* t_out) {
     // waited for, so the steps of small grids run side by side
     int first = OLLIN_OK;
     std::string first_msg;
+    Stepping stepping(n);
     for (int k = 0; k < n && first == OLLIN_OK; ++k) {
+        hs[k]->beside = stepping.beside;
         // side by side the evolutions fill the SMs: ordinary launches (a
         // chained successor's waiting blocks would take room from the others)
         g_chain_launch = n == 1 && hs[k]->chain;
@@ -3009,11 +3043,12 @@ int ollin_gpu_coarse_step_fused(ollin_handle* const* hs, int n, double* t_out, i
     //    is stepped on its own stream instead
     std::vector<LaunchRecorder> rec(n);
     std::vector<int> direct;
+    Stepping stepping(n);
     for (int k = 0; k < n; ++k) {
         ollin_handle* h = hs[k];
+        h->beside = stepping.beside;
         if (!h->sync.empty()) { direct.push_back(k); continue; }
         g_chain_launch = false;
-        rec[k].members = n;
         g_recorder = &rec[k];
         const int rc = onestep(h, 0);
         g_recorder = nullptr;

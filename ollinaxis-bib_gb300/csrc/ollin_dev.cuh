@@ -47,7 +47,6 @@ struct LaunchRec {
 };
 struct LaunchRecorder {
     std::vector<LaunchRec> recs;
-    int members = 1;  // evolutions of the call
 };
 extern thread_local LaunchRecorder* g_recorder;
 
@@ -188,17 +187,27 @@ __host__ __device__ inline size_t off(const LevelGeom& G, int i, int j) { return
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double ld_(const double* p) { return __ldg(p); }
 
+// the sums of the one-sided first differences at a line's end (s points
+// inwards) and one point from it, in order four, and at the end in order two
+__device__ __forceinline__ double at_end(const double* f, long s) {
+    return fma(3.0, ld_(f + 4 * s), fma(-16.0, ld_(f + 3 * s), fma(36.0, ld_(f + 2 * s), fma(-48.0, ld_(f + s), 25.0 * ld_(f)))));
+}
+__device__ __forceinline__ double one_in(const double* f, long s) {
+    return fma(6.0, ld_(f + 2 * s), fma(-18.0, ld_(f + s), fma(10.0, ld_(f), 3.0 * ld_(f - s)))) - ld_(f + 3 * s);
+}
+__device__ __forceinline__ double at_end2(const double* f, long s) { return fma(3.0, ld_(f), fma(-4.0, ld_(f + s), ld_(f + 2 * s))); }
+
 __device__ __forceinline__ double d1(const double* f, long s, int k, double c) {
     if (k == 0) {
         return c * (8.0 * (ld_(f + s) - ld_(f - s)) - (ld_(f + 2 * s) - ld_(f - 2 * s)));
     } else if (k == 1) {
-        return c * (3.0 * ld_(f + s) + 10.0 * ld_(f) - 18.0 * ld_(f - s) + 6.0 * ld_(f - 2 * s) - ld_(f - 3 * s));
+        return c * one_in(f, -s);
     } else if (k == 2) {
-        return c * (25.0 * ld_(f) - 48.0 * ld_(f - s) + 36.0 * ld_(f - 2 * s) - 16.0 * ld_(f - 3 * s) + 3.0 * ld_(f - 4 * s));
+        return c * at_end(f, -s);
     } else if (k == -1) {
-        return -c * (3.0 * ld_(f - s) + 10.0 * ld_(f) - 18.0 * ld_(f + s) + 6.0 * ld_(f + 2 * s) - ld_(f + 3 * s));
+        return -c * one_in(f, s);
     } else {
-        return -c * (25.0 * ld_(f) - 48.0 * ld_(f + s) + 36.0 * ld_(f + 2 * s) - 16.0 * ld_(f + 3 * s) + 3.0 * ld_(f + 4 * s));
+        return -c * at_end(f, s);
     }
 }
 
@@ -271,20 +280,20 @@ __device__ __forceinline__ double d2rz(const double* f, long ld, int i, int j, i
 // interior range (i = 3-ghost), 10 = n-2, 11 = n-1, 12 = n.
 __device__ __forceinline__ double dadv(const double* f, long s, int i, int n, int g, bool neg, double ih, bool zdir) {
     const double q = 0.25 * ih;
-    auto left = [&]() { return +q * (3.0 * ld_(f + s) + 10.0 * ld_(f) - 18.0 * ld_(f - s) + 6.0 * ld_(f - 2 * s) - ld_(f - 3 * s)) * (1.0 / 3.0); };
-    auto right = [&]() { return -q * (3.0 * ld_(f - s) + 10.0 * ld_(f) - 18.0 * ld_(f + s) + 6.0 * ld_(f + 2 * s) - ld_(f + 3 * s)) * (1.0 / 3.0); };
+    auto left = [&]() { return +q * one_in(f, -s) * (1.0 / 3.0); };
+    auto right = [&]() { return -q * one_in(f, s) * (1.0 / 3.0); };
     auto cent = [&]() { return q * (8.0 * (ld_(f + s) - ld_(f - s)) - (ld_(f + 2 * s) - ld_(f - 2 * s))) * (1.0 / 3.0); };
     if (i >= 4 - g && i <= n - 3) return neg ? left() : right();
     if (i == n - 2) return neg ? left() : cent();
     if (i == n - 1) return left();
-    if (i == n) return q * (25.0 * ld_(f) - 48.0 * ld_(f - s) + 36.0 * ld_(f - 2 * s) - 16.0 * ld_(f - 3 * s) + 3.0 * ld_(f - 4 * s)) * (1.0 / 3.0);
+    if (i == n) return q * at_end(f, -s) * (1.0 / 3.0);
     if (i == 3 - g) {
         // the r and z lopsided routines treat this point with opposite branches
         if (!zdir) return neg ? cent() : right();
         return neg ? right() : cent();
     }
     if (i == 2 - g) return right();
-    return -q * (25.0 * ld_(f) - 48.0 * ld_(f + s) + 36.0 * ld_(f + 2 * s) - 16.0 * ld_(f + 3 * s) + 3.0 * ld_(f + 4 * s)) * (1.0 / 3.0);
+    return -q * at_end(f, s) * (1.0 / 3.0);
 }
 
 // ---------------------------------------------------------------------------
@@ -297,8 +306,8 @@ __device__ __forceinline__ int pclass2(int i, int n, int g) { return i == n ? 2 
 
 __device__ __forceinline__ double d1_2(const double* f, long s, int k, double c) {
     if (k == 0) return c * (ld_(f + s) - ld_(f - s));
-    if (k == 2) return c * (3.0 * ld_(f) - 4.0 * ld_(f - s) + ld_(f - 2 * s));
-    return -c * (3.0 * ld_(f) - 4.0 * ld_(f + s) + ld_(f + 2 * s));
+    if (k == 2) return c * at_end2(f, -s);
+    return -c * at_end2(f, s);
 }
 
 __device__ __forceinline__ double d2_2(const double* f, long s, int k, double c) {
@@ -340,8 +349,8 @@ __device__ __forceinline__ double d2rz_2(const double* f, long ld, int i, int j,
 // every point alike
 __device__ __forceinline__ double dadv_2(const double* f, long s, int i, int n, int g, bool neg, double ih) {
     const double h = 0.5 * ih;
-    auto left = [&]() { return +h * (3.0 * ld_(f) - 4.0 * ld_(f - s) + ld_(f - 2 * s)); };
-    auto right = [&]() { return -h * (3.0 * ld_(f) - 4.0 * ld_(f + s) + ld_(f + 2 * s)); };
+    auto left = [&]() { return +h * at_end2(f, -s); };
+    auto right = [&]() { return -h * at_end2(f, s); };
     auto cent = [&]() { return h * (ld_(f + s) - ld_(f - s)); };
     if (i >= 3 - g && i <= n - 2) return neg ? left() : right();
     if (i == 2 - g) return neg ? cent() : right();

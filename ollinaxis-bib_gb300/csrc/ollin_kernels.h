@@ -75,6 +75,10 @@ struct StageArgs {
     int analysis;                // kAna* bits: write these quantities instead of updating
     int deldef;                  // DelDef (X_DELDEFR..X_GDZ) stands in aux; 0: formed here from g_A, g_B, g_C
     int rhs_blocks;              // blocks of the right-hand side's launch (set by the launcher)
+    // which kernel the launcher takes, and how it cuts its work (the results are
+    // the same bits): SMs of the device, evolutions being stepped, this one
+    // included, and those of them whose kernels run at the same time
+    int sms, beside, abreast;
     unsigned int* nanflag;       // set to 1 if a non-finite source is produced
     // The lapse of the level's last ``auxiliary`` call when a maximal-slicing
     // solve has replaced the lapse since (launch_rhs_stale, _stale_sync): the

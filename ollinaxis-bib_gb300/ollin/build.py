@@ -26,7 +26,9 @@ def nvcc():
 
 def _compile(src):
     obj = os.path.join(BUILD, os.path.splitext(src)[0] + ".o")
-    cmd = [nvcc()] + ARCH + COMMON + ["-c", os.path.join(CSRC, src), "-o", obj]
+    # the right-hand side's roundings are written out (rhs_kernel.cuh)
+    fmad = ["-fmad=false"] if src.startswith("rhs") else []
+    cmd = [nvcc()] + ARCH + COMMON + fmad + ["-c", os.path.join(CSRC, src), "-o", obj]
     if src.endswith(".cpp"):
         cmd = [nvcc()] + COMMON + ["-x", "cu"] + ARCH + ["-c", os.path.join(CSRC, src), "-o", obj]
     r = subprocess.run(cmd, capture_output=True, text=True)
