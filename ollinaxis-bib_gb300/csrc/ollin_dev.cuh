@@ -183,7 +183,8 @@ __host__ __device__ inline size_t off(const LevelGeom& G, int i, int j) { return
 // stride between consecutive points along the direction; ``k`` the position
 // class: 0 interior, 1 second-to-last, 2 last point (upper edge), -1 second
 // point, -2 first point (lower edge, used only without equatorial symmetry).
-// ``c`` is 1/(12 h) for first and 1/(12 h^2) for second derivatives.
+// ``c`` is 1/(12 h).  (Second and mixed derivatives and the dissipation are formed
+// in integers, rhs_stencil.cuh.)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double ld_(const double* p) { return __ldg(p); }
 
@@ -211,67 +212,10 @@ __device__ __forceinline__ double d1(const double* f, long s, int k, double c) {
     }
 }
 
-__device__ __forceinline__ double d2(const double* f, long s, int k, double c) {
-    if (k == 0) {
-        return -c * fma(30.0, ld_(f), fma(-16.0, ld_(f + s) + ld_(f - s), ld_(f + 2 * s) + ld_(f - 2 * s)));
-    } else if (k == 1) {
-        return c * (10.0 * ld_(f + s) - 15.0 * ld_(f) - 4.0 * ld_(f - s) + 14.0 * ld_(f - 2 * s) - 6.0 * ld_(f - 3 * s) + ld_(f - 4 * s));
-    } else if (k == 2) {
-        return c * (45.0 * ld_(f) - 154.0 * ld_(f - s) + 214.0 * ld_(f - 2 * s) - 156.0 * ld_(f - 3 * s) + 61.0 * ld_(f - 4 * s) - 10.0 * ld_(f - 5 * s));
-    } else if (k == -1) {
-        return c * (10.0 * ld_(f - s) - 15.0 * ld_(f) - 4.0 * ld_(f + s) + 14.0 * ld_(f + 2 * s) - 6.0 * ld_(f + 3 * s) + ld_(f + 4 * s));
-    } else {
-        return c * (45.0 * ld_(f) - 154.0 * ld_(f + s) + 214.0 * ld_(f + 2 * s) - 156.0 * ld_(f + 3 * s) + 61.0 * ld_(f + 4 * s) - 10.0 * ld_(f + 5 * s));
-    }
-}
-
 // Position class along one direction for first/second derivatives.
 __device__ __forceinline__ int pclass(int i, int n, int g) {
     if (i <= n - 2) return (i >= 3 - g) ? 0 : (i == 2 - g ? -1 : -2);
     return (i == n - 1) ? 1 : 2;
-}
-
-// Mixed derivative d^2/(dr dz) with the reference's edge and corner rules
-// (derivatives.f90:615-700): 4th order inside, 2nd order on the two outermost
-// rows/columns, one-sided on the last one, and the z-edge rule overriding the
-// r-edge rule where both apply.
-__device__ __forceinline__ double d2rz(const double* f, long ld, int i, int j, int nr, int nz, int g, double idrz) {
-    const bool ri = (i >= 3 - g && i <= nr - 2), zi = (j >= 3 - g && j <= nz - 2);
-#define F_(a, b) ld_(f + (a) + (long)(b) * ld)
-    if (ri && zi) {
-        return fma(idrz * (1.0 / 3.0), (F_(1, 1) + F_(-1, -1)) - (F_(1, -1) + F_(-1, 1)),
-                   (idrz * (-1.0 / 48.0)) * ((F_(2, 2) + F_(-2, -2)) - (F_(2, -2) + F_(-2, 2))));
-    }
-    const bool zedge_loop = (i >= 2 - g && i <= nr - 1);  // z-boundary loop range
-    const bool redge_loop = (j >= 2 - g && j <= nz - 1);  // r-boundary loop range
-    if (zedge_loop && !zi) {
-        if (j == 2 - g || j == nz - 1)
-            return 0.25 * idrz * (F_(1, 1) + F_(-1, -1) - F_(-1, 1) - F_(1, -1));
-        if (j == nz)
-            return 0.25 * idrz * ((3.0 * F_(1, 0) - 4.0 * F_(1, -1) + F_(1, -2)) - (3.0 * F_(-1, 0) - 4.0 * F_(-1, -1) + F_(-1, -2)));
-        // j == 1-g
-        return -0.25 * idrz * ((3.0 * F_(1, 0) - 4.0 * F_(1, 1) + F_(1, 2)) - (3.0 * F_(-1, 0) - 4.0 * F_(-1, 1) + F_(-1, 2)));
-    }
-    if (redge_loop && !ri) {
-        if (i == 2 - g || i == nr - 1)
-            return 0.25 * idrz * (F_(1, 1) + F_(-1, -1) - F_(1, -1) - F_(-1, 1));
-        if (i == nr)
-            return 0.25 * idrz * ((3.0 * F_(0, 1) - 4.0 * F_(-1, 1) + F_(-2, 1)) - (3.0 * F_(0, -1) - 4.0 * F_(-1, -1) + F_(-2, -1)));
-        return -0.25 * idrz * ((3.0 * F_(0, 1) - 4.0 * F_(1, 1) + F_(2, 1)) - (3.0 * F_(0, -1) - 4.0 * F_(1, -1) + F_(2, -1)));
-    }
-    // corners
-    if (i == nr && j == nz)
-        return 0.25 * idrz * (9.0 * F_(0, 0) + 16.0 * F_(-1, -1) + F_(-2, -2) - 12.0 * (F_(0, -1) + F_(-1, 0))
-                              + 3.0 * (F_(0, -2) + F_(-2, 0)) - 4.0 * (F_(-1, -2) + F_(-2, -1)));
-    if (i == nr)  // j == 1-g
-        return -0.25 * idrz * (9.0 * F_(0, 0) + 16.0 * F_(-1, 1) + F_(-2, 2) - 12.0 * (F_(0, 1) + F_(-1, 0))
-                               + 3.0 * (F_(0, 2) + F_(-2, 0)) - 4.0 * (F_(-1, 2) + F_(-2, 1)));
-    if (j == nz)  // i == 1-g
-        return -0.25 * idrz * (9.0 * F_(0, 0) + 16.0 * F_(1, -1) + F_(2, -2) - 12.0 * (F_(1, 0) + F_(0, -1))
-                               + 3.0 * (F_(2, 0) + F_(0, -2)) - 4.0 * (F_(2, -1) + F_(1, -2)));
-    return 0.25 * idrz * (9.0 * F_(0, 0) + 16.0 * F_(1, 1) + F_(2, 2) - 12.0 * (F_(0, 1) + F_(1, 0))
-                          + 3.0 * (F_(0, 2) + F_(2, 0)) - 4.0 * (F_(1, 2) + F_(2, 1)));
-#undef F_
 }
 
 // Lopsided advective derivative (src/base/derivadvect.f90, order four).
@@ -297,10 +241,9 @@ __device__ __forceinline__ double dadv(const double* f, long s, int i, int n, in
 }
 
 // ---------------------------------------------------------------------------
-// order two (derivatives.f90 :50-58, :158-172, :285-301, :402-418, :533-599;
-// derivadvect.f90 :50-100, :249-299; dissipation.f90 :121-135).  Position
-// classes: 0 centred (i = 2-ghost..n-1), 2 last point, -2 first point.
-// ``c`` is 1/(2h) for first and 1/h^2 for second derivatives.
+// order two (derivatives.f90 :50-58, :158-172; derivadvect.f90 :50-100,
+// :249-299).  Position classes: 0 centred (i = 2-ghost..n-1), 2 last point,
+// -2 first point.  ``c`` is 1/(2h).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int pclass2(int i, int n, int g) { return i == n ? 2 : (i >= 2 - g ? 0 : -2); }
 
@@ -308,41 +251,6 @@ __device__ __forceinline__ double d1_2(const double* f, long s, int k, double c)
     if (k == 0) return c * (ld_(f + s) - ld_(f - s));
     if (k == 2) return c * at_end2(f, -s);
     return -c * at_end2(f, s);
-}
-
-__device__ __forceinline__ double d2_2(const double* f, long s, int k, double c) {
-    if (k == 0) return c * (ld_(f + s) - 2.0 * ld_(f) + ld_(f - s));
-    if (k == 2) return c * (2.0 * ld_(f) - 5.0 * ld_(f - s) + 4.0 * ld_(f - 2 * s) - ld_(f - 3 * s));
-    return c * (2.0 * ld_(f) - 5.0 * ld_(f + s) + 4.0 * ld_(f + 2 * s) - ld_(f + 3 * s));
-}
-
-// centred inside, one-sided on the outermost rows and columns, the corners
-// from both one-sided stencils (the r- and z-edge loops do not overlap)
-__device__ __forceinline__ double d2rz_2(const double* f, long ld, int i, int j, int nr, int nz, int g, double idrz) {
-#define F_(a, b) ld_(f + (a) + (long)(b) * ld)
-    const bool ri = (i >= 2 - g && i <= nr - 1), zi = (j >= 2 - g && j <= nz - 1);
-    const double q = 0.25 * idrz;
-    if (ri && zi) return q * (F_(1, 1) + F_(-1, -1) - F_(1, -1) - F_(-1, 1));
-    if (zi) {  // i = 1-g or nr
-        if (i == nr) return q * ((3.0 * F_(0, 1) - 4.0 * F_(-1, 1) + F_(-2, 1)) - (3.0 * F_(0, -1) - 4.0 * F_(-1, -1) + F_(-2, -1)));
-        return -q * ((3.0 * F_(0, 1) - 4.0 * F_(1, 1) + F_(2, 1)) - (3.0 * F_(0, -1) - 4.0 * F_(1, -1) + F_(2, -1)));
-    }
-    if (ri) {  // j = 1-g or nz
-        if (j == nz) return q * ((3.0 * F_(1, 0) - 4.0 * F_(1, -1) + F_(1, -2)) - (3.0 * F_(-1, 0) - 4.0 * F_(-1, -1) + F_(-1, -2)));
-        return -q * ((3.0 * F_(1, 0) - 4.0 * F_(1, 1) + F_(1, 2)) - (3.0 * F_(-1, 0) - 4.0 * F_(-1, 1) + F_(-1, 2)));
-    }
-    if (i == nr && j == nz)
-        return q * (9.0 * F_(0, 0) + 16.0 * F_(-1, -1) + F_(-2, -2) - 12.0 * (F_(0, -1) + F_(-1, 0))
-                    + 3.0 * (F_(0, -2) + F_(-2, 0)) - 4.0 * (F_(-1, -2) + F_(-2, -1)));
-    if (i == nr)
-        return -q * (9.0 * F_(0, 0) + 16.0 * F_(-1, 1) + F_(-2, 2) - 12.0 * (F_(0, 1) + F_(-1, 0))
-                     + 3.0 * (F_(0, 2) + F_(-2, 0)) - 4.0 * (F_(-1, 2) + F_(-2, 1)));
-    if (j == nz)
-        return -q * (9.0 * F_(0, 0) + 16.0 * F_(1, -1) + F_(2, -2) - 12.0 * (F_(1, 0) + F_(0, -1))
-                     + 3.0 * (F_(2, 0) + F_(0, -2)) - 4.0 * (F_(2, -1) + F_(1, -2)));
-    return q * (9.0 * F_(0, 0) + 16.0 * F_(1, 1) + F_(2, 2) - 12.0 * (F_(0, 1) + F_(1, 0))
-                + 3.0 * (F_(0, 2) + F_(2, 0)) - 4.0 * (F_(1, 2) + F_(2, 1)));
-#undef F_
 }
 
 // second-order lopsided advective derivative; the r and z routines treat
@@ -359,45 +267,14 @@ __device__ __forceinline__ double dadv_2(const double* f, long s, int i, int n, 
     return left();  // i == n
 }
 
-// the fourth difference of order-two dissipation (without -eps/dt/6)
-__device__ __forceinline__ double ko4(const double* f, long s) {
-    return 6.0 * ld_(f) - 4.0 * (ld_(f + s) + ld_(f - s)) + (ld_(f + 2 * s) + ld_(f - 2 * s));
-}
-
 // ---- order dispatch for the kernels that take the order at run time ------
 __device__ __forceinline__ int pclass_o(int ord, int i, int n, int g) { return ord == 2 ? pclass2(i, n, g) : pclass(i, n, g); }
 __device__ __forceinline__ double c1_o(int ord, double ih) { return ord == 2 ? 0.5 * ih : ih * (1.0 / 12.0); }
-__device__ __forceinline__ double c2_o(int ord, double ih) { return ord == 2 ? ih * ih : ih * ih * (1.0 / 12.0); }
 __device__ __forceinline__ double d1_o(int ord, const double* f, long s, int k, double c) {
     return ord == 2 ? d1_2(f, s, k, c) : d1(f, s, k, c);
-}
-__device__ __forceinline__ double d2_o(int ord, const double* f, long s, int k, double c) {
-    return ord == 2 ? d2_2(f, s, k, c) : d2(f, s, k, c);
-}
-__device__ __forceinline__ double d2rz_o(int ord, const double* f, long ld, int i, int j, int nr, int nz, int g, double idrz) {
-    return ord == 2 ? d2rz_2(f, ld, i, j, nr, nz, g, idrz) : d2rz(f, ld, i, j, nr, nz, g, idrz);
 }
 // the first point whose r derivative diff1r sets: i = 1 in order four,
 // i = 2-ghost in order two (lower points of a grid off the axis stay unset)
 __device__ __forceinline__ int d1r_first(int ord, int g) { return ord == 2 ? 2 - g : 1; }
-
-// Kreiss-Oliger sixth difference along one direction, the bracket of
-// src/base/dissipation.f90:196-211 (without the -eps/dt/20 factor).
-__device__ __forceinline__ double ko6(const double* f, long s) {
-    return 20.0 * ld_(f) - 15.0 * (ld_(f + s) + ld_(f - s)) + 6.0 * (ld_(f + 2 * s) + ld_(f - 2 * s)) - (ld_(f + 3 * s) + ld_(f - 3 * s));
-}
-
-// s - k * (ko6 along stride 1 + ko6 along stride ld), for points inside both
-// dissipation ranges: the two brackets share the centre and are summed
-// before scaling (13 FP64 operations instead of 16).
-__device__ __forceinline__ double ko6rz_apply(const double* f, long ld, double k, double s) {
-    const double a1 = (ld_(f + 1) + ld_(f - 1)) + (ld_(f + ld) + ld_(f - ld));
-    const double a2 = (ld_(f + 2) + ld_(f - 2)) + (ld_(f + 2 * ld) + ld_(f - 2 * ld));
-    const double a3 = (ld_(f + 3) + ld_(f - 3)) + (ld_(f + 3 * ld) + ld_(f - 3 * ld));
-    double t = fma(-40.0 * k, ld_(f), s);
-    t = fma(15.0 * k, a1, t);
-    t = fma(-6.0 * k, a2, t);
-    return fma(k, a3, t);
-}
 
 }  // namespace ollin
