@@ -49,7 +49,9 @@ def cost(e):
         return c
     if e.is_Add:
         c = sum(cost(a) for a in e.args) + len(e.args) - 1
-        fus = sum(1 for a in e.args if a.is_Mul and (len(a.args) >= 2))
+        # a product takes the addition in; -a is not one
+        fus = sum(1 for a in e.args if a.is_Pow or a.is_Mul and not (
+            len(a.args) == 2 and a.args[0] == -1 and not a.args[1].is_Pow))
         return c - min(fus, len(e.args) - 1)
     return sum(cost(a) for a in e.args)
 

@@ -9,10 +9,10 @@
 // than the unit reaches (a factor of 16, of 4 at the ends of a line: in some 8%
 // of the warps' lines next to a puncture, 25% in the tails of a shell), the sum
 // of what was cut off is added, and where they are 2^25 (2^23) apart, smaller
-// than 2^-895 or not finite (under 1% of the lines of a shell), the sums are
-// formed in FP64.  So a difference is nowhere further from its exact value than
+// than 2^-895 or not finite (far out in a shell's tails, on coarse grids), the
+// sums are formed in FP64.  So a difference is nowhere further from its exact value than
 // FP64 has it (the shell exp(-(r-5)^2) for r from 8 to 16 with h = 0.25: first
-// difference to 2e-16 of its value, second to 1e-16; in FP64 8e-16 and 5e-15;
+// difference to 2e-16 of its value, second to 3e-16; in FP64 8e-16 and 5e-15;
 // with neighbours cut at the unit 4e-14 and 1e-13).  A field's five derivatives,
 // advection and dissipation take some 700 integer instructions instead of 45 FP64
 // ones of 64-76 clocks each, and leave the FP64 unit to the pointwise algebra.
